@@ -63,7 +63,9 @@ const char* rijk_status_string(int status);
 int rijk_ctx_info(const rijk_ctx* ctx, int64_t* num_basis, int64_t* num_auxbas, int64_t* tensor_bytes);
 /* The context's CUDA stream (a cudaStream_t). */
 void* rijk_ctx_stream(rijk_ctx* ctx);
-/* Device pointer of the tile-packed tensor and its row stride in doubles. */
+/* Device pointer of the tile-packed tensor and its row stride in doubles; for
+ * reading (rows are written by rijk_tensor_load_rows_dev, which keeps what the
+ * library derives from them up to date). */
 int rijk_ctx_tensor(rijk_ctx* ctx, const double** d_tensor, int64_t* row_stride);
 /* Number of CUDA kernels this library has launched in this process (all
  * contexts); a caller can difference it around a region to count launches. */
@@ -140,7 +142,10 @@ int rijk_get_rimatr(rijk_ctx* ctx, double* rimatr);
 /* Tensors produced on the device (e.g. by a device integral engine): allocate a
  * zero tensor for (num_basis, num_auxbas), then load aux rows [p0, p0+np) from
  * device memory, rimatr rows (layout 0, npair doubles each) or ri3fn blocks
- * (layout 1, n*n doubles each).  Same roles as rijk_set_rimatr/_ri3fn. */
+ * (layout 1, n*n doubles each).  Same roles as rijk_set_rimatr/_ri3fn.  A load is
+ * enqueued on `stream` and may also go to a pinned context: what runs behind it in
+ * stream order, replays of captured FP64 builds included, sees the new rows (a
+ * captured split-precision build has to be captured again). */
 int rijk_tensor_alloc(rijk_ctx* ctx, int64_t num_basis, int64_t num_auxbas);
 int rijk_tensor_load_rows_dev(rijk_ctx* ctx, const double* d_rows, int64_t p0, int64_t np, int layout,
                               void* stream);

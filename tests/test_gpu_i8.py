@@ -201,3 +201,88 @@ def test_group_of_both_forms():
     g.close()
     for c in ctxs:
         c.close()
+
+
+@pytest.mark.parametrize("n,naux,o", [(130, 37, 21), (260, 21, 140)])
+def test_captured_build_follows_the_tensor(n, naux, o):
+    """A build captured on a pinned context and replayed after other rows were loaded
+    into the tensor: some a thousand times larger than the ones it was captured with,
+    some zero before."""
+    import torch
+
+    old, new = host_case(n, naux, o, seed=1), host_case(n, naux, o, seed=2)
+    r0 = old.rimatr.copy(order="F")
+    r0[:, naux // 2:] = 0.0
+    r1 = np.asfortranarray(1000.0 * new.rimatr)
+    c = torch.as_tensor(old.c_occ.T.copy(), device="cuda")
+    occ = torch.full((o,), 2.0, dtype=torch.float64, device="cuda")
+    dm = 2.0 * c.T @ c
+    rows = torch.as_tensor(r1.T.copy(), device="cuda")
+    npair = n * (n + 1) // 2
+
+    def build(ctx, out):
+        st = torch.cuda.current_stream().cuda_stream
+        ctx.vjk_upper_occ_dev(c.data_ptr(), o, [o - 1], occ.data_ptr(), 1, 1.0, 1.0, out[0].data_ptr(),
+                              out[1].data_ptr(), st)
+        ctx.vk_upper_dm_dev(dm.data_ptr(), 1, 1.0, out[2].data_ptr(), st)
+
+    want, got = (torch.zeros(3, npair, dtype=torch.float64, device="cuda") for _ in range(2))
+    with _ctx(r1, n) as fresh:
+        build(fresh, want)
+        fresh.synchronize(torch.cuda.current_stream().cuda_stream)
+    with _ctx(r0, n) as ctx:
+        build(ctx, got)
+        torch.cuda.synchronize()
+        ctx.pin_buffers(True)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            build(ctx, got)
+        st = torch.cuda.current_stream().cuda_stream
+        ctx.tensor_load_rows_dev(rows.data_ptr(), 0, naux, 0, st)
+        graph.replay()
+        ctx.synchronize(st)
+        # the same kernels on the same operands, their K partials and J shares added in one order
+        assert torch.equal(got, want)
+        del graph
+        ctx.pin_buffers(False)
+
+
+def test_every_producer_of_the_tensor():
+    """Each way a tensor gets into a context, after one of much smaller elements, gives
+    the same K: what the INT8 form keeps of the rows is the new tensor's."""
+    import torch
+
+    n, naux, o = 72, 40, 9
+    case = host_case(n, naux, o, seed=6)
+    full = np.asfortranarray(_full(case.rimatr, n).transpose(1, 2, 0))
+    rows = torch.as_tensor(np.ascontiguousarray(case.rimatr.T), device="cuda")
+    blocks = torch.as_tensor(np.ascontiguousarray(full.transpose(2, 1, 0)), device="cuda")
+    torch.cuda.synchronize()
+    eye = np.eye(naux, order="F")
+
+    def by_rows(ctx):
+        ctx.tensor_alloc(n, naux)
+        ctx.tensor_load_rows_dev(rows.data_ptr(), 0, 17, 0)
+        ctx.tensor_load_rows_dev(blocks[17:].data_ptr(), 17, naux - 17, 1)
+
+    producers = [lambda ctx: ctx.set_rimatr(case.rimatr, n), lambda ctx: ctx.set_ri3fn(full), by_rows,
+                 lambda ctx: ctx.fit_rimatr(eye, case.rimatr, n),
+                 lambda ctx: ctx.build_rimatr_cholesky(eye, case.rimatr, n)]
+    got = []
+    for produce in producers:
+        with _ctx(np.asfortranarray(1e-6 * case.rimatr), n) as ctx:
+            produce(ctx)
+            got.append(_k(ctx, n, [case.c_occ], [np.ones(o)])[0])
+    for k in got[1:]:
+        assert np.array_equal(k, got[0])
+
+    from rest_b200.geometry import water_cluster
+
+    mol = water_cluster(3, seed=1)
+    bas, aux = mol.shells("def2-SVP"), mol.shells("def2-SVP-JKFIT")
+    with _ctx(np.asfortranarray(1e-6 * case.rimatr), n) as ctx:
+        ctx.build_rimatr_from_shells(bas, aux)
+        k = _k(ctx, n, [case.c_occ], [np.ones(o)])[0]
+        r = ctx.get_rimatr()
+    with _ctx(r, n) as ctx:
+        assert np.array_equal(k, _k(ctx, n, [case.c_occ], [np.ones(o)])[0])
