@@ -832,7 +832,8 @@ def device_bytes(n: int, naux: int, nocc: int, precision: str = "fp64") -> int:
     ldx = -(-n // 128) * 128
     scratch = min(4 << 30, naux * ldx * (-(-nocc // 128) * 128) * 8)
     split = naux_pad * ldx * ldx * 4 if precision in ("mixed", "split") else 0
-    # the grouped build's half-transform scratch: X, its digits, the tensor rows' maxima
+    # the grouped build's half-transform scratch, X and its digits, and the context's
+    # maxima of the tensor rows
     group = naux * nocc * ldx * 15 + naux * ldx * 4
     return tensor + scratch + split + group + 8 * n * n * 8
 

@@ -286,3 +286,38 @@ def test_every_producer_of_the_tensor():
         r = ctx.get_rimatr()
     with _ctx(r, n) as ctx:
         assert np.array_equal(k, _k(ctx, n, [case.c_occ], [np.ones(o)])[0])
+
+
+def test_group_created_behind_loads_in_flight():
+    """Rows are loaded, a group made of their context and a build enqueued, all on one
+    non-blocking stream that is still busy: stream order alone has to be enough."""
+    import torch
+
+    from rest_b200 import RIJK, RIJKGroup
+
+    n, naux, o = 150, 60, 20
+    case = host_case(n, naux, o, seed=9)
+    with _ctx(case.rimatr, n) as ctx:
+        vj, vk = ctx.vjk_upper_with_ri_v([case.c_occ], [o - 1], [np.full(o, 2.0)], 1, 1.0, -0.5)
+    rows = torch.as_tensor(np.ascontiguousarray(case.rimatr.T), device="cuda")
+    C = torch.as_tensor(np.ascontiguousarray(case.c_occ), device="cuda")
+    active = torch.ones(1, dtype=torch.int32, device="cuda")
+    out = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+    busy = torch.randn(4096, 4096, device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with RIJK(0) as ctx:
+        ctx.tensor_alloc(n, naux)
+        with torch.cuda.stream(st):
+            x = busy
+            for _ in range(40):  # some tens of milliseconds
+                x = (x @ busy) * 1e-2
+        ctx.tensor_load_rows_dev(rows.data_ptr(), 0, naux, 0, st.cuda_stream)
+        g = RIJKGroup([ctx], [o])
+        g.jk_occ_dev(C.data_ptr(), n * o, o, 1, -0.5, active.data_ptr(), out.data_ptr(), n * n, n, st.cuda_stream)
+        g.synchronize(st.cuda_stream)
+        g.close()
+    jj, ii = np.tril_indices(n)
+    ref = vj[0] + vk[0]
+    # both sum naux o products and naux rows in FP64, in other orders
+    assert np.abs(out.cpu().numpy()[ii, jj] - ref).max() <= 1e-12 * np.abs(ref).max()
