@@ -7,6 +7,9 @@
 namespace rijk {
 
 constexpr int I8_DIGITS = 7;  // base-256 digits of an operand
+// A level sums at most seven digit products of 2^14 per element of the contracted index:
+// this many stay below 2^31 (the half-transform contracts over the basis functions).
+constexpr int64_t I8_MAX_N = 16384;
 
 // `active` of the launches below: null, or a device flag; where it is 0 the kernel
 // does nothing (a group's converged molecules in a captured graph).

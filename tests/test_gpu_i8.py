@@ -321,3 +321,30 @@ def test_group_created_behind_loads_in_flight():
     ref = vj[0] + vk[0]
     # both sum naux o products and naux rows in FP64, in other orders
     assert np.abs(out.cpu().numpy()[ii, jj] - ref).max() <= 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [16384, 27000])
+def test_largest_sums_of_the_half_transform(n):
+    """Every digit of both operands at the end of its range, over the most functions the
+    INT8 form takes and over more than 32-bit sums of such products hold (18808 for
+    digits 0 and 6 together with 1 and 5, 2 and 4, 3 and 3; what overflows at 27000 is
+    of weight 2^-29 of the sum, far above the tolerance)."""
+    import torch
+
+    from rest_b200 import RIJK
+
+    b = -(126 * 256**6 + 128 * (256**6 - 1) // 255) / 2.0**55
+    npair = n * (n + 1) // 2
+    rows = torch.full((npair,), b, dtype=torch.float64, device="cuda")
+    c = torch.full((n,), b, dtype=torch.float64, device="cuda")
+    occ = torch.ones(1, dtype=torch.float64, device="cuda")
+    vj, vk = (torch.empty(npair, dtype=torch.float64, device="cuda") for _ in range(2))
+    st = torch.cuda.current_stream().cuda_stream
+    with RIJK(0) as ctx:
+        ctx.tensor_alloc(n, 1)
+        ctx.tensor_load_rows_dev(rows.data_ptr(), 0, 1, 0, st)
+        ctx.vjk_upper_occ_dev(c.data_ptr(), 1, [0], occ.data_ptr(), 1, 1.0, 1.0, vj.data_ptr(), vk.data_ptr(), st)
+        ctx.synchronize(st)
+    for out, ref in ((vk, (n * b * b) ** 2), (vj, n * n * b**4)):  # X = n b c; w = sum of n x c, J = w B
+        # sums of n equal terms, then products: n + 3 roundings
+        assert float((out - ref).abs().max()) <= (n + 3) * 2.0**-53 * abs(ref)
