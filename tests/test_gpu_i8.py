@@ -348,3 +348,37 @@ def test_largest_sums_of_the_half_transform(n):
     for out, ref in ((vk, (n * b * b) ** 2), (vj, n * n * b**4)):  # X = n b c; w = sum of n x c, J = w B
         # sums of n equal terms, then products: n + 3 roundings
         assert float((out - ref).abs().max()) <= (n + 3) * 2.0**-53 * abs(ref)
+
+
+def test_threads_of_different_sizes():
+    """Contexts of several host threads load rows at once: what one of them sets up
+    for its kernels does not depend on another's size."""
+    import threading
+
+    import torch
+
+    from rest_b200 import RIJK
+
+    errors = []
+    sizes = (64, 1200, 130, 1000)
+    rows = torch.zeros(1200 * 1201 // 2, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ready = threading.Barrier(len(sizes))
+
+    def work(n):
+        try:
+            with RIJK(0) as ctx:
+                ctx.tensor_alloc(n, 1)
+                ready.wait()
+                for _ in range(3000):
+                    ctx.tensor_load_rows_dev(rows.data_ptr(), 0, 1, 0, 0)
+                ctx.synchronize()
+        except Exception as e:  # noqa: BLE001 (reported by the test)
+            errors.append((n, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
