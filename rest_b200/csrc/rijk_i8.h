@@ -28,9 +28,9 @@ int i8_rank_splits(int64_t n, int64_t k, int full);
 // Kpart[split][q] (128 x 128 blocks q over block pairs, as launch_k_rank_update
 // writes them) = the split's share of X Y^T for the digit matrices X and Y (ldx
 // rows, k columns each; xmax and ymax their rows' maxima, as maxhi above).  full = 0: the
-// blocks' upper triangle only.  False when the operands' tensor maps could not be encoded
-// (nothing is launched and the error flag is set).
-void launch_i8_rank(int64_t n, int64_t ldx, int64_t k, const int8_t* xdig, const int* xmax, const int8_t* ydig,
+// blocks' upper triangle only.  False when the operands' tensor maps could not be encoded:
+// nothing is launched then.
+bool launch_i8_rank(int64_t n, int64_t ldx, int64_t k, const int8_t* xdig, const int* xmax, const int8_t* ydig,
                     const int* ymax, int splits, int full, double* Kpart, int* err, cudaStream_t st,
                     const int* active = nullptr);
 
@@ -77,8 +77,9 @@ struct I8Next {
 void launch_i8_max_rows(const int* bmax, int64_t ldx, int64_t np, int* cmax, cudaStream_t st);
 int64_t i8_row_bytes(int64_t nt, int64_t ldx);
 int64_t i8_chunk_rows(const I8Cols& c, int64_t nt, int64_t ldx, int64_t naux, int64_t bytes);
-// xmax[spin ldx + row] takes the high word of the largest |X[row, :]| (the caller clears it)
-void launch_i8_half(const I8Cols& c, int64_t n, int64_t nt, int64_t ldx, int64_t ldB, const I8Chunk& cur,
+// xmax[spin ldx + row] takes the high word of the largest |X[row, :]| (the caller clears it).
+// False as launch_i8_rank's.
+bool launch_i8_half(const I8Cols& c, int64_t n, int64_t nt, int64_t ldx, int64_t ldB, const I8Chunk& cur,
                     const I8Next& next, const double* Cw, const int8_t* digits, const double* factor, int* xmax, int* err,
                     cudaStream_t st, const int* active = nullptr);
 // per-warp shares of J's scalars per aux row, for launch_j_wreduce
