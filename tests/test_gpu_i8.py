@@ -382,3 +382,19 @@ def test_threads_of_different_sizes():
     for t in threads:
         t.join()
     assert not errors
+
+
+@pytest.mark.parametrize("up", [980, -980])
+def test_operands_at_the_ends_of_the_range(up):
+    """Tensor and orbitals scaled against each other: X is the unscaled problem's."""
+    n, naux, o = 140, 9, 11
+    case = host_case(n, naux, o, seed=5)
+    x = np.einsum("pmn,ni->mpi", _full(case.rimatr, n), case.c_occ).reshape(n, -1)
+    r = np.asfortranarray(np.ldexp(case.rimatr, up))
+    c = np.asfortranarray(np.ldexp(case.c_occ, -up))
+    with _ctx(r, n) as ctx:
+        k = _k(ctx, n, [c], [np.ones(o)])[0]
+    # as test_k_within_the_operands_rounding
+    m = np.abs(x).max(axis=1)
+    bscale = np.abs(case.rimatr).max() * np.abs(case.c_occ).max()
+    assert np.abs(k - x @ x.T).max() <= 2 * naux * o * (m.max() ** 2 + n * m.max() * bscale) * 2.0**-53
