@@ -85,6 +85,23 @@ enum rijk_prof_class {
   RIJK_PROF_K_OTHER = 6,    /* operand preparation, reduction   */
   RIJK_PROF_NCLASS = 7
 };
+/* Arithmetic of the exchange contractions (no counterpart in REST, whose BLAS sums in
+ * FP64).  RIJK_EXCHANGE_INT8, the default, runs them from 64 basis functions on (density
+ * form from 128, group members from 120) on the INT8 tensor cores: each row of B_P, column
+ * of C or D and row of the half-transformed X is held to 55 bits below its own largest
+ * element.  The error of an element of X, K, or J from the same half-transform, is that of
+ * FP64 sums of the same length relative to the product of its two rows' (its row's and
+ * column's) norms; measured over a whole J or K it is no larger than DMMA's.  It is not
+ * that of FP64 sums relative to the element's own terms: where all of those are far below
+ * the norms (localised orbitals, a sparse density) fewer digits of the element are
+ * significant.  def2-SVP K of (H2O)16 and C20H42, largest error over the sum of the terms'
+ * magnitudes: eigenvectors of the density 3e-14 (DMMA 4e-15), its Cholesky vectors 2e-10
+ * (1e-14), density form 3e-10 (1e-14); in norm 2e-15, 2e-15, 2e-15 (2e-15, 4e-15, 3e-15).
+ * RIJK_EXCHANGE_DMMA runs every size on the FP64 tensor cores, whose error is relative to
+ * each element's own terms, at about half the speed.  Takes effect at the next build, in
+ * groups at their creation. */
+enum rijk_exchange_form { RIJK_EXCHANGE_INT8 = 0, RIJK_EXCHANGE_DMMA = 1 };
+int rijk_ctx_set_exchange(rijk_ctx* ctx, int form);
 /* CTA shapes of the DMMA K kernels, which small molecules, ao2mo and the small
  * members of a group use (larger ones run on the INT8 tensor cores, whose tiles are
  * fixed; results agree to rounding across them), for

@@ -70,6 +70,7 @@ SIGNATURES = {
     "rijk_ctx_set_tiles": (C.c_int, [_ctxp, C.c_int, C.c_int]),
     "rijk_ctx_get_tiles": (C.c_int, [_ctxp, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "rijk_ctx_pin_buffers": (C.c_int, [_ctxp, C.c_int]),
+    "rijk_ctx_set_exchange": (C.c_int, [_ctxp, C.c_int]),
     "rijk_ctx_set_wait_budget": (C.c_int, [_ctxp, C.c_int64]),
     "rijk_group_create": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
     "rijk_group_destroy": (C.c_int, [C.c_void_p]),

@@ -113,6 +113,16 @@ class RIJK:
         """Freeze the context's device memory (for CUDA graph capture of *_dev calls)."""
         self._check(lib().rijk_ctx_pin_buffers(self._h, int(bool(pinned))))
 
+    EXCHANGE_FORMS = {"int8": 0, "dmma": 1}
+
+    def set_exchange(self, form: str = "int8"):
+        """Arithmetic of the exchange contractions: "int8" (55 bits below each row's
+        largest element, on the INT8 tensor cores) or "dmma" (FP64 tensor cores at
+        every size: each element accurate relative to its own terms)."""
+        if form not in self.EXCHANGE_FORMS:
+            raise ValueError(f"exchange form must be one of {sorted(self.EXCHANGE_FORMS)}")
+        self._check(lib().rijk_ctx_set_exchange(self._h, self.EXCHANGE_FORMS[form]))
+
     def set_wait_budget(self, nanoseconds: int = 0):
         """Budget of every device-side wait of this context (0 = default 2 s)."""
         self._check(lib().rijk_ctx_set_wait_budget(self._h, int(nanoseconds)))

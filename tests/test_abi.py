@@ -84,3 +84,7 @@ def test_int8_launchers_report_operands_without_a_tensor_map(L):
     assert fn(C.byref(cols), n, C.c_int64(5), ldx, C.c_int64(15 * 1024), C.byref(Chunk(np=4)), C.byref(Next()), None,
               None, None, None, C.byref(err), None, None) is False
     assert err.value == 0
+
+
+def test_exchange_form_needs_a_context(L):
+    assert L.rijk_ctx_set_exchange(None, 0) == 1

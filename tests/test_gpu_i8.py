@@ -398,3 +398,72 @@ def test_operands_at_the_ends_of_the_range(up):
     m = np.abs(x).max(axis=1)
     bscale = np.abs(case.rimatr).max() * np.abs(case.c_occ).max()
     assert np.abs(k - x @ x.T).max() <= 2 * naux * o * (m.max() ** 2 + n * m.max() * bscale) * 2.0**-53
+
+
+def _local_case(n, naux, seed):
+    """A tensor whose elements fall off with the functions' distance, to 1e-50."""
+    rng = np.random.default_rng(seed)
+    pos = rng.uniform(0, 20, (n, 3))
+    env = np.exp(-0.1 * ((pos[:, None] - pos[None]) ** 2).sum(-1))
+    s = np.exp(np.log(1e-3) * rng.uniform(size=naux))
+    jj, ii = np.tril_indices(n)
+    return np.asfortranarray((rng.standard_normal((naux, ii.size)) * s[:, None] * env[ii, jj]).T), rng
+
+
+def test_exchange_form_is_the_callers_choice():
+    """Orbitals on one function each, so that many elements of K have only terms far
+    below the rows' largest: DMMA's error is relative to those terms, the INT8 form's to
+    the rows' maxima."""
+    import torch
+
+    from rest_b200 import RIJKGroup
+
+    n, naux, o = 200, 60, 33
+    r, rng = _local_case(n, naux, 0)
+    b = _full(r, n)
+    c = np.zeros((n, o), order="F")
+    c[rng.choice(n, o, replace=False), np.arange(o)] = 1.0
+    d = np.asfortranarray(np.diag(rng.uniform(0.5, 1.0, n)))
+    x = np.einsum("pmn,ni->mpi", b, c).reshape(n, -1)
+    t = (b @ d).transpose(1, 0, 2).reshape(n, -1)
+    y = b.transpose(1, 0, 2).reshape(n, -1)
+    jj, ii = np.tril_indices(n)
+    with _ctx(r, n) as ctx:
+        with pytest.raises(ValueError):
+            ctx.set_exchange("fp32")
+        for form in ("int8", "dmma"):
+            ctx.set_exchange(form)
+            k = _k(ctx, n, [c], [np.ones(o)])[0]
+            kd = ctx.vk_full_fromdm_with_ri_v([d], 1, 1.0)[0]
+            # X is exact (one term an element), K sums naux o products, twice (the
+            # reference's own rounding); T one product, K naux n
+            for got, p, q, terms in ((k, x, x, naux * o), (kd, t, y, naux * n)):
+                err = np.abs(got - p @ q.T)
+                own = 2 * (terms + 1) * 2.0**-53 * (np.abs(p) @ np.abs(q).T)
+                if form == "dmma":
+                    assert np.all(err <= own)
+                else:
+                    # digits: 2^-54 of the rows' maxima for B, X (or T) and B each,
+                    # through naux o (naux n) products
+                    top = np.abs(y).max(axis=1)
+                    assert np.all(err <= own + 8 * terms * 2.0**-53 * np.outer(top, top))
+                    assert np.any(err > 1e3 * own)  # what the other form is there for
+        # a group takes each member's choice at creation
+        C = torch.as_tensor(np.ascontiguousarray(c), device="cuda")
+        active = torch.ones(1, dtype=torch.int32, device="cuda")
+        out = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        vj = ctx.vj_upper_with_rimatr_v([np.asfortranarray(2.0 * c @ c.T)], 1, 1.0)[0]
+        g = RIJKGroup([ctx], [o])
+        ctx.set_exchange("int8")
+        g.jk_occ_dev(C.data_ptr(), n * o, o, 1, 1.0, active.data_ptr(), out.data_ptr(), n * n, n)
+        g.synchronize()
+        g.close()
+        ref = 2 * x @ x.T
+        jf = np.zeros((n, n))
+        jf[ii, jj] = jf[jj, ii] = vj
+        own = (np.abs(ref) + np.abs(jf)) + 2 * np.abs(x) @ np.abs(x).T
+        # J's terms: naux scalars of o n products each, times the tensor's elements
+        w = 2 * np.einsum("pmn,mi,ni->p", np.abs(b), np.abs(c), np.abs(c))
+        own = own + np.einsum("p,pmn->mn", w, np.abs(b))
+        assert np.all(np.abs(out.cpu().numpy() - ref - jf) <= 2 * naux * n * 2.0**-53 * own)
