@@ -286,6 +286,10 @@ typedef struct rijk_group rijk_group;
 int rijk_group_create(rijk_ctx* const* ctxs, int count, const int64_t* nocc, int half_transform_cfg, int update_cfg,
                       rijk_group** out);
 int rijk_group_destroy(rijk_group* group);
+/* The form (RIJK_EXCHANGE_*) in which a group created now would build ctx's molecule
+ * with nocc occupied orbitals: the CTA shapes apply to DMMA members only, so an
+ * autotuner has to time one of those. */
+int rijk_group_member_exchange(const rijk_ctx* ctx, int64_t nocc);
 /* For every molecule m with d_active[m] != 0 (device int array):
  *   out_m = J(D_m) + k_scale K(C_m),  D_m = 2 C_m C_m^T over the nocc[m] columns,
  * written full and symmetric (n_m x n_m) at d_out + m out_mol with row stride ldo;

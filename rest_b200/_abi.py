@@ -74,6 +74,7 @@ SIGNATURES = {
     "rijk_ctx_set_wait_budget": (C.c_int, [_ctxp, C.c_int64]),
     "rijk_group_create": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_void_p)]),
     "rijk_group_destroy": (C.c_int, [C.c_void_p]),
+    "rijk_group_member_exchange": (C.c_int, [_ctxp, C.c_int64]),
     "rijk_group_jk_occ_dev": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_double,
                                         C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),
     "rijk_group_synchronize": (C.c_int, [C.c_void_p, C.c_void_p]),

@@ -123,6 +123,11 @@ class RIJK:
             raise ValueError(f"exchange form must be one of {sorted(self.EXCHANGE_FORMS)}")
         self._check(lib().rijk_ctx_set_exchange(self._h, self.EXCHANGE_FORMS[form]))
 
+    def group_exchange(self, nocc: int) -> str:
+        """The form in which a group would build this molecule with ``nocc`` orbitals."""
+        form = lib().rijk_group_member_exchange(self._h, int(nocc))
+        return next(k for k, v in self.EXCHANGE_FORMS.items() if v == form)
+
     def set_wait_budget(self, nanoseconds: int = 0):
         """Budget of every device-side wait of this context (0 = default 2 s)."""
         self._check(lib().rijk_ctx_set_wait_budget(self._h, int(nanoseconds)))
@@ -411,6 +416,7 @@ def group_tiles(ctx: "RIJK", nocc: int, sample_rows: int = 256):
     """The project's autotuner applied to a group: times every CTA shape on
     ``ctx``'s tensor (rijk_ctx_autotune) and keeps the fastest of those the
     grouped build supports, for the half-transform and for the rank update.
+    The shapes are the DMMA members' (``ctx.group_exchange``): pass one of those.
     The choice is kept per molecule shape for the rest of the process, so that
     repeated runs take the same summation order, and ``ctx``'s own shapes are
     left as they were."""

@@ -142,16 +142,19 @@ class BatchedRHF:
         with host_blas_limit(host_blas_threads):
             self._setup(mols, basis, auxbas, device, metric, integrals, setup_workers, contexts)
         # Grouped FP64 build: every molecule's J + K in one set of launches
-        # (rijk_group_*), tile shapes from the autotuner on the largest molecule,
-        # captured once in a CUDA graph and replayed every iteration.  It serves
+        # (rijk_group_*), tile shapes from the autotuner on the largest molecule
+        # that takes them (larger ones run on the INT8 tensor cores), captured once in a CUDA graph and replayed every iteration.  It serves
         # every build when no molecule takes split-precision steps.
         self._group, self._ggraph = None, None
         self.group_graphs = group_graphs
         all_fp64 = precision == "fp64" or (precision == "mixed" and max(self.n) < split_min_basis)
         if grouped and all_fp64:
             t0 = time.perf_counter()
-            big = max(range(self.B), key=lambda i: self.n[i])
-            tiles = group_tiles(self.ctx[big], self.nocc[big], sample_rows=256)
+            dmma = [i for i in range(self.B) if self.ctx[i].group_exchange(self.nocc[i]) == "dmma"]
+            tiles = ()  # the default shapes, which no member uses
+            if dmma:
+                big = max(dmma, key=lambda i: self.n[i])
+                tiles = group_tiles(self.ctx[big], self.nocc[big], sample_rows=256)
             self._group = RIJKGroup(self.ctx, self.nocc, *tiles)
             self.setup_parts["group"] = time.perf_counter() - t0
             self.setup_s += self.setup_parts["group"]

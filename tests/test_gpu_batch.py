@@ -279,3 +279,20 @@ def test_grouped_batch_equals_per_molecule_batch():
     assert all(res[True].converged) and all(res[False].converged)
     for a, b in zip(res[True].energies, res[False].energies):
         assert abs(a - b) < 1e-9
+
+
+@pytest.mark.parametrize("waters,tuned", [((1, 4, 6), 4), ((5, 6), None)])
+def test_group_shapes_are_timed_on_a_member_that_takes_them(monkeypatch, waters, tuned):
+    """From 120 functions on (five waters) a member runs on the INT8 tensor cores, whose
+    tiles are fixed: the shapes come from the largest of the others, if there is one."""
+    from rest_b200 import scf_batch
+
+    seen = []
+    tiles = scf_batch.group_tiles
+    monkeypatch.setattr(scf_batch, "group_tiles",
+                        lambda ctx, nocc, **kw: (seen.append(ctx.shape()[0] // 24), tiles(ctx, nocc, **kw))[1])
+    b = BatchedRHF([water_cluster(k, seed=k) for k in waters], "def2-SVP", "def2-SVP-JKFIT", precision="fp64")
+    try:
+        assert seen == ([tuned] if tuned else [])
+    finally:
+        b.close()
