@@ -467,3 +467,48 @@ def test_exchange_form_is_the_callers_choice():
         w = 2 * np.einsum("pmn,mi,ni->p", np.abs(b), np.abs(c), np.abs(c))
         own = own + np.einsum("p,pmn->mn", w, np.abs(b))
         assert np.all(np.abs(out.cpu().numpy() - ref - jf) <= 2 * naux * n * 2.0**-53 * own)
+
+
+def test_digits_of_the_update():
+    """K_ij = o x_i x_j of operands with all seven digits in use, against whole numbers:
+    the update from X (orbitals on one function each, so that X is the tensor's columns)
+    and from T and the tensor's rows (the density form with D = 1)."""
+    import i8_cases as I
+
+    n, o = 170, 8
+    pat = I.patterns(n - o, 3)
+    v = [I.value(d) for d in pat]
+    b = np.zeros((1, n, n))
+    b[0, o:, :o] = np.array(v, dtype=float)[:, None]
+    b[0, :o, o:] = b[0, o:, :o].T
+    jj, ii = np.tril_indices(n)
+    c = np.asfortranarray(np.eye(n)[:, :o])
+    with _ctx(np.asfortranarray(b[:, ii, jj].T), n) as ctx:
+        k = _k(ctx, n, [c], [np.ones(o)])[0]
+        kd = ctx.vk_full_fromdm_with_ri_v([np.asfortranarray(np.eye(n))], 1, 1.0)[0]
+    for got in (k, kd):  # all nonzero terms in one step of one split: a single rounding
+        for i in range(n - o):
+            for j in range(0, n - o, 7):
+                assert I.relative_error(got[o + i, o + j], o * v[i] * v[j]) <= I.PRODUCT_TOL
+
+
+@pytest.mark.parametrize("n,o", [(70, 1), (130, 17), (130, 130), (260, 200)])
+def test_digits_of_the_half_transform(n, o):
+    """X = n b c with all digits of b and c in use, seen through K = X X^T: digits made in
+    the tile and through memory, in the first and the last column of the orbitals."""
+    import i8_cases as I
+
+    pat = I.patterns(4, n)
+    jj, ii = np.tril_indices(n)
+    for db in pat:
+        b = I.value(db)
+        with _ctx(np.full((ii.size, 1), float(b), order="F"), n) as ctx:
+            for dc in pat[:3]:
+                for col in {0, o - 1}:
+                    c = np.zeros((n, o), order="F")
+                    c[:, col] = float(I.value(dc))
+                    k = _k(ctx, n, [c], [np.ones(o)])[0]
+                    x = int(float(n * b * I.value(dc)))  # rounded to nearest, as the levels' sum is
+                    # X one rounding off at most (the dropped levels turn a tie), twice in K
+                    err = max(I.relative_error(k[i, j], x * x) for i in (0, 31, 32, n // 2, n - 1) for j in (0, n - 1))
+                    assert err <= 2 * 2.0**-53 + I.PRODUCT_TOL
