@@ -12,7 +12,8 @@ constexpr int I8_DIGITS = 7;  // base-256 digits of an operand
 constexpr int64_t I8_MAX_N = 16384;
 
 // `active` of the launches below: null, or a device flag; where it is 0 the kernel
-// does nothing (a group's converged molecules in a captured graph).
+// does nothing (a group's converged molecules in a captured graph).  Groups take the
+// in-tile half-transform only, and only that form of launch_i8_half looks at it.
 
 // Digits of a column-major FP64 matrix X (ldx rows, ldx a multiple of 128, k
 // columns): for every group of 16 columns, digit and row the 16 digits of that

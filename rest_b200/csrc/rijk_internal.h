@@ -26,11 +26,12 @@ void count_launch(int64_t k = 1);
 int64_t launch_count();
 
 // --- layout conversion -------------------------------------------------------
-// rimatr (REST MatrixFull[npair, N], column P = packed upper of B_P), rows
-// [p0, p0 + np) -> tile-packed rows [p0, p0 + np) of dB.
-void launch_pack_rimatr(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st);
-// ri3fn (REST RIFull[n,n,N]), aux rows [p0, p0+np): upper triangle is the source.
-void launch_pack_ri3fn(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st);
+// np aux rows of src -> tile-packed rows at dst.  src_kind 0: rimatr (REST
+// MatrixFull[npair, N], column P = packed upper of B_P); 1: ri3fn (REST
+// RIFull[n,n,N]), whose upper triangle is the source.  bmax: null, or takes each
+// row's largest magnitudes (high words, ldx per aux row), for the INT8 exchange.
+void launch_pack(const Geom& g, const double* src, int src_kind, int64_t np, double* dst, int* bmax, int64_t ldx,
+                 cudaStream_t st);
 // tile-packed rows -> rimatr rows.
 void launch_unpack_rimatr(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st);
 

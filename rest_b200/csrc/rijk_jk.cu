@@ -44,12 +44,24 @@ __device__ __forceinline__ int64_t tri_root(int64_t t) {
 // ============================================================================
 // One CTA per stored tile (blockIdx.x), aux rows strided over blockIdx.y.
 // src_kind 0: rimatr rows (npair each); 1: ri3fn blocks (n*n each).
+// bmax (zeroed by the caller) or null: bmax[p ldx + mu] takes the high word of the
+// largest |B_p[mu, :]|, from the elements in registers: 46 aux rows of n = 1200 take 132 us
+// without, 139 with, some 500 where a pass of its own reads them back.
 __global__ void __launch_bounds__(256) k_pack(int64_t n, int64_t npair, int64_t ldB, const double* __restrict__ src,
-                                              int src_kind, int64_t np, double* __restrict__ dst) {
+                                              int src_kind, int64_t np, double* __restrict__ dst,
+                                              int* __restrict__ bmax, int64_t ldx) {
+  __shared__ int m[2 * TS];  // the tile's rows, then its columns
   const int64_t t = blockIdx.x;
   const int64_t J = tri_root(t), I = t - J * (J + 1) / 2;
+  const int tid = threadIdx.x;
   for (int64_t p = blockIdx.y; p < np; p += gridDim.y) {
-    for (int e = threadIdx.x; e < TILE_ELEMS; e += blockDim.x) {
+    int row = 0;
+    if (bmax) {
+      __syncthreads();  // m of the aux row before is read
+      if (tid < 2 * TS) m[tid] = 0;
+      __syncthreads();
+    }
+    for (int e = tid; e < TILE_ELEMS; e += 256) {
       const int r = e & 31, c = e >> 5;
       const int64_t mu = I * TS + r, nu = J * TS + c;
       double v = 0.0;
@@ -58,6 +70,19 @@ __global__ void __launch_bounds__(256) k_pack(int64_t n, int64_t npair, int64_t 
         v = src_kind == 0 ? src[p * npair + packed_upper_index(i, j)] : src[p * n * n + i + n * j];
       }
       dst[p * ldB + t * TILE_ELEMS + e] = v;
+      if (bmax) {
+        const int h = __double2hiint(v) & 0x7fffffff;
+        row = max(row, h);
+        const int col = __reduce_max_sync(0xffffffffu, h);
+        if (r == 0) m[TS + c] = col;  // a warp has a column to itself
+      }
+    }
+    if (bmax) {
+      atomicMax(&m[tid & 31], row);
+      __syncthreads();
+      // (a diagonal tile holds both triangles: its rows are enough)
+      if (tid < (I == J ? TS : 2 * TS) && m[tid] > 0)
+        atomicMax(bmax + p * ldx + (tid < TS ? I * TS + tid : J * TS + tid - TS), m[tid]);
     }
   }
 }
@@ -74,17 +99,13 @@ __global__ void __launch_bounds__(256) k_unpack_rimatr(int64_t n, int64_t npair,
   }
 }
 
-void launch_pack_rimatr(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st) {
+void launch_pack(const Geom& g, const double* src, int src_kind, int64_t np, double* dst, int* bmax, int64_t ldx,
+                 cudaStream_t st) {
   if (np <= 0) return;
   dim3 grid((unsigned)g.ntp, (unsigned)std::min<int64_t>(np, 65535));
+  if (bmax) cudaMemsetAsync(bmax, 0, (size_t)np * ldx * sizeof(int), st);
   count_launch();
-  k_pack<<<grid, 256, 0, st>>>(g.n, g.npair, g.ldB, src, 0, np, dst);
-}
-void launch_pack_ri3fn(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st) {
-  if (np <= 0) return;
-  dim3 grid((unsigned)g.ntp, (unsigned)std::min<int64_t>(np, 65535));
-  count_launch();
-  k_pack<<<grid, 256, 0, st>>>(g.n, g.npair, g.ldB, src, 1, np, dst);
+  k_pack<<<grid, 256, 0, st>>>(g.n, g.npair, g.ldB, src, src_kind, np, dst, bmax, ldx);
 }
 void launch_unpack_rimatr(const Geom& g, const double* src, int64_t np, double* dst, cudaStream_t st) {
   if (np <= 0) return;
