@@ -326,6 +326,32 @@ def run_ours(args, w):
                  "what": "J by two passes over the tensor (rijk_vj_upper_dev) + K (rijk_vk_upper_occ_dev)"
                  if args.jk == "fused" else "rijk_vjk_upper_occ_dev"}
 
+    # the exchange's other arithmetic on the same workload (for the record)
+    exchange = {"form": "int8", "what": "FP64 operands as seven INT8 digits (55 bits below each row's largest "
+                f"element), {INT8_PRODUCTS} exact digit products on tcgen05, their sums added in FP64; "
+                "rijk_ctx_set_exchange chooses the FP64 tensor cores instead"}
+    if not args.no_split:
+        step()
+        ctx.synchronize(st)
+        vj_i8, vk_i8 = vj.clone(), vk.clone()
+        ctx.set_exchange("dmma")
+        for _ in range(2):
+            step()
+        torch.cuda.synchronize()
+        d0, d1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        d0.record(stream)
+        for _ in range(3):
+            step()
+        d1.record(stream)
+        torch.cuda.synchronize()
+        t_dmma = d0.elapsed_time(d1) / 1e3 / 3
+        exchange.update({"dmma_ms_per_step": t_dmma * 1e3, "dmma_value": world * flops / t_dmma / 1e12,
+                         "j_rel_diff_norm": float((vj - vj_i8).norm() / vj.norm()),
+                         "k_rel_diff_norm": float((vk - vk_i8).norm() / vk.norm())})
+        ctx.set_exchange("int8")
+        step()
+        del vj_i8, vk_i8
+
     # split-precision exchange (3 x BF16 on tcgen05) on the same workload: the
     # first call builds the BF16 copies of the tensor (once per geometry)
     split = None
@@ -512,6 +538,7 @@ def run_ours(args, w):
             "cpu_baseline": cpu_base,
             "jk_form": args.jk,
             "other_jk_form": other,
+            "exchange": exchange,
             "split_precision": split,
             "scf_water": scf,
             **apps,

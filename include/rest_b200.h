@@ -276,7 +276,8 @@ int rijk_vjk_upper_lowrank_split_dev(rijk_ctx* ctx, const double* d_V, int64_t l
  * 2490-2561, 2758-2834); a group runs that build for many molecules (one
  * context each, tensors loaded) in six launches for all of them, the two
  * tensor-core phases as persistent kernels over work items (molecule, aux row,
- * tile); J's aux-row scalars come out of the half-transform phase, so J reads
+ * tile); members that run on the INT8 tensor cores take five kernels and a memset of
+ * their own in place of those two phases.  J's aux-row scalars come out of the half-transform phase, so J reads
  * each tensor once.  nocc[m]: doubly occupied orbitals of molecule m.  The CTA shapes are
  * 0, 1 or 4 of rijk_ctx_set_tiles (the caller's autotuner picks them).  The
  * group owns the scratch of all molecules (one allocation at creation); its

@@ -11,8 +11,9 @@ stream), and the SCF iterations of the whole set advance together:
                overlap the others' device work;
   J / K        FP64 builds of a group of molecules (``grouped``) by the
                library's grouped build (rijk_group_jk_occ_dev: six launches for
-               all of them, captured once in a CUDA graph and replayed every
-               iteration with the converged molecules switched off); otherwise
+               all of them and six more for each INT8 member, captured once in a
+               CUDA graph and replayed every iteration with the converged
+               molecules switched off); otherwise
                per molecule through the device entry points
                (rijk_vjk_upper_occ_dev, which takes J from the K half-transform,
                or the split-precision tcgen05 forms), the molecules' launches
@@ -34,7 +35,7 @@ stream), and the SCF iterations of the whole set advance together:
   density      D = 2 C_occ C_occ^T on the device.
 
 Precision of the exchange build:
-  fp64   every K in FP64 (DMMA, from 64 basis functions on exact INT8 digit products);
+  fp64   every K in FP64 (DMMA, from 64 basis functions on INT8 digits of 55 bits);
   mixed  for molecules with at least ``split_min_basis`` (512) basis functions,
          incremental split-precision J and K: K_k = K_{k-1} + K_split(D_k - D_{k-1})
          and J_k = J_{k-1} + J(D_k - D_{k-1}), J's aux-row scalars taken from the
