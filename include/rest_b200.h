@@ -98,8 +98,9 @@ enum rijk_prof_class {
  * magnitudes: eigenvectors of the density 3e-14 (DMMA 4e-15), its Cholesky vectors 2e-10
  * (1e-14), density form 3e-10 (1e-14); in norm 2e-15, 2e-15, 2e-15 (2e-15, 4e-15, 3e-15).
  * RIJK_EXCHANGE_DMMA runs every size on the FP64 tensor cores, whose error is relative to
- * each element's own terms, at about half the speed.  Takes effect at the next build, in
- * groups at their creation. */
+ * each element's own terms, at about half the speed; a build or a group whose INT8 scratch
+ * does not fit the device takes it, too.  Takes effect at the next build, in groups at
+ * their creation. */
 enum rijk_exchange_form { RIJK_EXCHANGE_INT8 = 0, RIJK_EXCHANGE_DMMA = 1 };
 int rijk_ctx_set_exchange(rijk_ctx* ctx, int form);
 /* CTA shapes of the DMMA K kernels, which small molecules, ao2mo and the small

@@ -512,3 +512,70 @@ def test_digits_of_the_half_transform(n, o):
                     # X one rounding off at most (the dropped levels turn a tie), twice in K
                     err = max(I.relative_error(k[i, j], x * x) for i in (0, 31, 32, n // 2, n - 1) for j in (0, n - 1))
                     assert err <= 2 * 2.0**-53 + I.PRODUCT_TOL
+
+
+def _leave_free(nbytes):
+    """Device memory held so that about ``nbytes`` stay free."""
+    import torch
+    from cuda.bindings import runtime
+
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    # what the stream-ordered pool keeps would come back to an allocation that fails
+    err, pool = runtime.cudaDeviceGetDefaultMemPool(torch.cuda.current_device())
+    assert int(err) == 0 and int(runtime.cudaMemPoolTrimTo(pool, 0)[0]) == 0
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(free - nbytes, dtype=torch.uint8, device="cuda")
+
+
+def test_builds_without_room_for_the_digits():
+    """With room for the DMMA form's scratch only, a build and a group take that form
+    (half-transformed orbitals or density 1.2, 0.5 and 2.6 GB; the digits' form 1.6, 1.3
+    and 4.9)."""
+    import torch
+
+    from rest_b200 import RIJK, RIJKGroup
+
+    for n, naux, o, free, kind in ((300, 2000, 200, 1400 << 20, "occ"), (300, 390, 200, 800 << 20, "dm"),
+                                   (130, 20000, 64, 3500 << 20, "group")):
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(n)
+        rows = torch.randn(naux // 10, n * (n + 1) // 2, generator=gen, dtype=torch.float64, device="cuda")
+        C = torch.linalg.qr(torch.randn(n, o, generator=gen, dtype=torch.float64, device="cuda"))[0].contiguous()
+        c = C.T.contiguous()
+        dm = C @ c
+        occ = torch.full((o,), 2.0, dtype=torch.float64, device="cuda")
+        vj, vk = (torch.empty(n * (n + 1) // 2, dtype=torch.float64, device="cuda") for _ in range(2))
+        active = torch.ones(1, dtype=torch.int32, device="cuda")
+        out = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        got = []
+        for short in (False, True):
+            with RIJK(0) as ctx:
+                ctx.tensor_alloc(n, naux)
+                for p in range(10):
+                    ctx.tensor_load_rows_dev(rows.data_ptr(), p * (naux // 10), naux // 10, 0)
+                ctx.synchronize()
+                launches = RIJK.kernel_launches()
+                hold = _leave_free(free) if short else None
+                if kind == "group":
+                    g = RIJKGroup([ctx], [o])
+                    g.jk_occ_dev(C.data_ptr(), n * o, o, 1, -0.5, active.data_ptr(), out.data_ptr(), n * n, n)
+                    g.synchronize()
+                    g.close()
+                    res = out.clone()
+                elif kind == "dm":
+                    ctx.vk_upper_dm_dev(dm.data_ptr(), 1, -0.5, vk.data_ptr())
+                    ctx.synchronize()
+                    res = vk.clone()
+                else:
+                    ctx.vjk_upper_occ_dev(c.data_ptr(), o, [o - 1], occ.data_ptr(), 1, 1.0, -0.5, vj.data_ptr(),
+                                          vk.data_ptr())
+                    ctx.synchronize()
+                    res = torch.stack([vj, vk])
+                del hold
+                torch.cuda.empty_cache()
+                got.append((res, RIJK.kernel_launches() - launches))
+        assert got[0][1] != got[1][1]  # the other form's launches
+        # both sum naux o products of sums of n, in other orders
+        assert float((got[1][0] - got[0][0]).abs().max()) <= 1e-12 * float(got[0][0].abs().max())
